@@ -249,9 +249,9 @@ int lsb_tau_sgs(lsb_handle* h, const double* ui, const double* uiuj, const doubl
  * that cannot pay for cudaMalloc/cudaFree's device-wide synchronisation.  No handle is
  * needed and nothing is allocated: every pointer is a device address the caller owns
  * (rhs, out: spectral (nx, ny, nzp); lam: nzm; e, ei: nzm x nzm row-major; wavx: nx;
- * wavy: ny), and the work memory is a static device array of LSB_NOALLOC_SCRATCH_BYTES
- * that every GPU loading the library keeps until exit.  Limit: nzp <= 129 (any nx*ny;
- * columns are processed in chunks that fit the array); larger nz returns
+ * wavy: ny), and the matrices' padded copies live in a static device array of LSB_NOALLOC_SCRATCH_BYTES
+ * that every GPU loading the library keeps until exit.  Limit: nzp <= 129 (any nx*ny);
+ * larger nz returns
  * LSB_ERR_UNSUPPORTED.  The first call on a device looks up the array's address, so make
  * it before any stream capture.  Calls share the array: calls that overlap on the GPU
  * race and must be serialised by the caller.  stream is a cudaStream_t of the current
@@ -259,7 +259,7 @@ int lsb_tau_sgs(lsb_handle* h, const double* ui, const double* uiuj, const doubl
  * found on the first call is kept for the life of the process: a device reset
  * (cudaDeviceReset, or the primary context destroyed and made again) is not supported
  * afterwards. */
-#define LSB_NOALLOC_SCRATCH_BYTES (8u << 20)
+#define LSB_NOALLOC_SCRATCH_BYTES (256u << 10)
 int lsb_solve_helmholtz_noalloc(int nx, int ny, int nz, const double* rhs, double* out, const double* lam,
                                 const double* e, const double* ei, const double* wavx, const double* wavy,
                                 double dtnui, void* stream);

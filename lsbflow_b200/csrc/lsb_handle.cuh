@@ -59,7 +59,7 @@ struct lsb_handle {
     double *hb = nullptr, *ht = nullptr, *d2hb = nullptr, *d2ht = nullptr, *lam = nullptr, *lamx = nullptr;
     std::vector<double> h_xpts, h_ypts, h_zpts, h_ubar;
     double dx = 0, dy = 0;
-    lsb::Mat m_dz1, m_dz2, m_dz2rows, m_ei, m_eext;
+    lsb::Mat m_dz1, m_dz2, m_dz2rows, m_ei, m_e, m_eext;
     // FFT plans: y (ny), y padded (nyl), x real (nx), x real padded (nxl)
     lsb::FftPlan py, pyl;
     lsb::RealPlan rx, rxl;

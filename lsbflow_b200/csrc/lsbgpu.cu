@@ -271,7 +271,14 @@ void helmholtz(lsb_handle* h, const double* rhs, double* out, int nf, double sig
     }
     // both contractions on the FP64 tensor cores: one launch, the intermediate in registers
     const bool fp64 = !(h->cfg.precision == 1 && tc);
-    if (fp64 && launch_helm_fused(g1, g2, h->stream)) return;
+    if (fp64) {
+        GemmArgs ge = g2;  // E without its zero boundary rows: the kernel writes those itself
+        ge.A = h->m_e.p;
+        ge.M = h->m_e.M;
+        ge.Mp = h->m_e.Mp;
+        ge.roff = 1;
+        if (launch_helm_fused(g1, ge, h->stream)) return;
+    }
     contract(h, g1, tc ? h->oz_ei : OzMat{});
     contract(h, g2, tc ? h->oz_eext : OzMat{});
 }
@@ -1289,6 +1296,7 @@ int lsb_create(const lsb_config* cfg, const lsb_setup* su, lsb_handle** out) {
             h->m_dz2rows = make_mat(h.get(), rows.data(), 2, nzp);
         }
         h->m_ei = make_mat(h.get(), su->ei, nzm, nzm);
+        h->m_e = make_mat(h.get(), su->e, nzm, nzm);
         h->m_eext = make_mat(h.get(), su->e, nzm, nzm, 0, nzm, 1, nzp);  // zero ceiling / wall rows
         if (cfg->precision == 1) {
             // the mixed form's contractions on the int8 tensor cores: D, E^-1 and E (the latter
