@@ -534,9 +534,31 @@ void launch_row_c2r(const RowJobList& jobs, const RowArgs& a, cudaStream_t s) {
     else { lsb::note_launch(); k_row_c2r<false><<<persistent_grid(k_row_c2r<false>, sm, nitems), 256, sm, s>>>(jobs, a); }
 }
 
+static void launch_row_r2c_batched(const RowJobList& jobs, const RowArgs& a, cudaStream_t s);
 void launch_row_r2c(const RowJobList& jobs, const RowArgs& a, cudaStream_t s) {
     if (jobs.n <= 0) return;
+    // Rows with the fringe factor (RowIO::lam) of the lengths that only the FP64 register plans
+    // cover stay with k_row_r2c, which transforms them WITHOUT the factor: a defect of that kernel
+    // (N then takes q instead of lambda (m - q)), older than those plans.  It is kept because
+    // correcting it changes the results of these lengths; the correction is to drop this split
+    // (the warp kernels apply the factor) and to give k_row_r2c the factor for the lengths left.
+    if (a.rp.half.fp64_only) {
+        RowJobList with{}, without{};
+        for (int i = 0; i < jobs.n; ++i) {
+            RowJobList& l = jobs.j[i].lam != nullptr ? with : without;
+            l.j[l.n++] = jobs.j[i];
+        }
+        if (with.n > 0) {
+            launch_row_r2c_batched(with, a, s);
+            launch_row_r2c(without, a, s);
+            return;
+        }
+    }
     if (launch_row_r2c_warp(jobs, a, s)) return;
+    launch_row_r2c_batched(jobs, a, s);
+}
+
+static void launch_row_r2c_batched(const RowJobList& jobs, const RowArgs& a, cudaStream_t s) {
     if (a.f32) throw std::runtime_error("mixed precision: x transform length has no warp plan");
     const int nitems = jobs.n * ((a.nyl * a.nzp + RB - 1) / RB);
     const size_t sm = (size_t)3 * RB * a.rp.half.ls * sizeof(double2);

@@ -7,7 +7,8 @@
 // G-point decimation-in-frequency network across the group's lanes with shfl_xor.  Lane g
 // ends with X[k1 + R*bitrev(g)] in register k1.  Shared memory is only used to turn the
 // strided/bit-reversed orders into coalesced global accesses; there is no block barrier
-// inside a transform.  Lengths whose R is not in {1,2,3,4,6,8} use fft_kernels.cu.
+// inside a transform.  Lengths whose R is not in {1,2,3,4,6,8}, or in FP64 {5,7,9,12,15}, use
+// fft_kernels.cu.
 #include <stdexcept>
 
 #include <cstring>
@@ -28,9 +29,7 @@ __device__ __forceinline__ int brev(int g, int lgg) {
     return lgg ? (int)(__brev((unsigned)g) >> (32 - lgg)) : 0;
 }
 
-// SEL = true: the butterflies as a per-lane select of both branches (fewer live registers,
-// more arithmetic; the FP64 product rows use it to stay within their register budget)
-template <int R, int SIGN, bool SEL = false, class V>
+template <int R, int SIGN, class V>
 __device__ __forceinline__ void wfft(V (&v)[R], int G, int g, const V* __restrict__ tw) {
     dft_reg<R, SIGN>(v);
     if (R > 1 && g != 0) {
@@ -52,17 +51,6 @@ __device__ __forceinline__ void wfft(V (&v)[R], int G, int g, const V* __restric
         const bool up = (g & h) != 0;
         V w = __ldg(&tw[j * st]);
         if (SIGN > 0) w.y = -w.y;
-        if (SEL) {
-#pragma unroll
-            for (int k1 = 0; k1 < R; ++k1) {
-                V o;
-                o.x = __shfl_xor_sync(0xffffffffu, v[k1].x, h);
-                o.y = __shfl_xor_sync(0xffffffffu, v[k1].y, h);
-                v[k1] = up ? cmul(csub(o, v[k1]), w) : cadd(v[k1], o);
-            }
-            st <<= 1;
-            continue;
-        }
         if (!up) w = CT<V>::make((S)1, (S)0);
         const S sg = up ? (S)-1 : (S)1;
 #pragma unroll
@@ -80,7 +68,7 @@ __device__ __forceinline__ void wfft(V (&v)[R], int G, int g, const V* __restric
 // Inverse of the order produced by wfft: input "slot" layout (lane g' register k1 holds
 // z[k1 + R*bitrev(g')]), cross-lane decimation-in-time network, twiddles, R-point DFT in
 // registers; output in natural order (lane g register r holds X[g + G*r]).
-template <int R, int SIGN, bool SEL = false, class V>
+template <int R, int SIGN, class V>
 __device__ __forceinline__ void wfft_dit(V (&v)[R], int G, int g, const V* __restrict__ tw) {
     // butterfly of the pair (g, g ^ h): the lower lane keeps v + w o, the upper o - w v.  The
     // upper lane multiplies its own value by w before the exchange (the lower lane's factor is
@@ -93,17 +81,6 @@ __device__ __forceinline__ void wfft_dit(V (&v)[R], int G, int g, const V* __res
         const bool up = (g & h) != 0;
         V w = __ldg(&tw[j * st]);
         if (SIGN > 0) w.y = -w.y;
-        if (SEL) {
-#pragma unroll
-            for (int k1 = 0; k1 < R; ++k1) {
-                V o;
-                o.x = __shfl_xor_sync(0xffffffffu, v[k1].x, h);
-                o.y = __shfl_xor_sync(0xffffffffu, v[k1].y, h);
-                v[k1] = up ? csub(o, cmul(w, v[k1])) : cadd(v[k1], cmul(w, o));
-            }
-            st >>= 1;
-            continue;
-        }
         if (!up) w = CT<V>::make((S)1, (S)0);
         const S sg = up ? (S)-1 : (S)1;
 #pragma unroll
@@ -139,8 +116,10 @@ __device__ __forceinline__ void lane_bitrev(V (&v)[R], int G, int lane, int g, i
     }
 }
 
-// Exchange networks for lane groups of G = 16 or 32 lanes with an even register count
-// R = 2H.  In the lane-pair networks above both lanes of a pair evaluate a butterfly branch
+// Exchange networks for lane groups of G = 4 .. 32 lanes with an even register count
+// R = 2H, or an odd one with one dummy register more (R' = R + 1 = 2H: the dummy's column never
+// meets another; 9 of 10 registers do useful butterflies where the lane-pair network evaluates
+// 18 branches).  In the lane-pair networks above both lanes of a pair evaluate a butterfly branch
 // for every register.  Here, at each stage, a lane sends half of its registers to its partner
 // and receives the partner's matching half, so that it holds H whole butterflies: half the
 // shuffles and half the butterfly arithmetic per stage.  Invariant before the stage on lane
@@ -151,13 +130,18 @@ __device__ __forceinline__ void lane_bitrev(V (&v)[R], int G, int lane, int g, i
 // whose next bit is set), and lanes with bit G/2 set start with their halves rotated.
 // DIF (wfft_x): dft_reg, twiddles, rotation, stages h = G/2 .. 1.  Lane g, register k then
 // holds X[m], m = xslot<R, G>(g, k) = k%H + H*g_top + R*bitrev(g mod G/2) + (N/2)*(k/H)
-// with N = R G and g_top the lane's bit G/2 -- the lane bit reversal of wfft is not needed.
+// with N = R G and g_top the lane's bit G/2 -- the lane bit reversal of wfft is not needed; with
+// odd R the column k%H + H*g_top = R of the upper half-group's last registers is the dummy (-1).
 // DIT (wfft_dit_x): the conjugate transpose of that network (stages h = 1 .. G/2, the
 // butterfly s +- w d, the data routing inverted), from that layout to natural order.
+__host__ __device__ constexpr int xregs(int R) { return R + R % 2; }
+
 template <int R, int G>
 __device__ __forceinline__ int xslot(int g, int k) {
-    constexpr int H = R / 2, LG = ilog2c(G);
-    return (k % H) + H * ((g >> (LG - 1)) & 1) + R * brev(g & (G / 2 - 1), LG - 1) + (G / 2) * R * (k / H);
+    constexpr int H = xregs(R) / 2, LG = ilog2c(G);
+    const int col = (k % H) + H * ((g >> (LG - 1)) & 1);
+    if (R % 2 == 1 && col == R) return -1;
+    return col + R * brev(g & (G / 2 - 1), LG - 1) + (G / 2) * R * (k / H);
 }
 
 template <int R, class V>
@@ -171,11 +155,27 @@ __device__ __forceinline__ void rotate_halves(V (&v)[R], bool on) {
     }
 }
 
+// the R-point DFT of the first R of RR registers
+template <int R, int SIGN, int RR, class V>
+__device__ __forceinline__ void dft_first(V (&v)[RR]) {
+    if constexpr (R == RR) {
+        dft_reg<R, SIGN>(v);
+    } else {
+        V u[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) u[r] = v[r];
+        dft_reg<R, SIGN>(u);
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = u[r];
+    }
+}
+
 template <int R, int SIGN, int G, class V>
-__device__ __forceinline__ void wfft_x(V (&v)[R], int g, const V* __restrict__ tw) {
-    static_assert(R % 2 == 0 && (G == 16 || G == 32), "exchange network: even R, 16- or 32-lane groups");
-    constexpr int H = R / 2;
-    dft_reg<R, SIGN>(v);
+__device__ __forceinline__ void wfft_x(V (&v)[xregs(R)], int g, const V* __restrict__ tw) {
+    static_assert(G >= 4 && G <= 32, "exchange network: 4- to 32-lane groups");
+    using S = typename CT<V>::S;
+    constexpr int RR = xregs(R), H = RR / 2;
+    dft_first<R, SIGN>(v);
     if (g != 0) {
 #pragma unroll
         for (int k1 = 1; k1 < R; ++k1) {
@@ -184,7 +184,8 @@ __device__ __forceinline__ void wfft_x(V (&v)[R], int g, const V* __restrict__ t
             v[k1] = cmul(v[k1], w);
         }
     }
-    rotate_halves<R>(v, (g & (G / 2)) != 0);
+    if (R % 2 == 1) v[RR - 1] = CT<V>::make((S)0, (S)0);
+    rotate_halves<RR>(v, (g & (G / 2)) != 0);
     int st = R;
 #pragma unroll
     for (int h = G / 2; h >= 1; h >>= 1) {
@@ -207,9 +208,9 @@ __device__ __forceinline__ void wfft_x(V (&v)[R], int g, const V* __restrict__ t
 }
 
 template <int R, int SIGN, int G, class V>
-__device__ __forceinline__ void wfft_dit_x(V (&v)[R], int g, const V* __restrict__ tw) {
-    static_assert(R % 2 == 0 && (G == 16 || G == 32), "exchange network: even R, 16- or 32-lane groups");
-    constexpr int H = R / 2;
+__device__ __forceinline__ void wfft_dit_x(V (&v)[xregs(R)], int g, const V* __restrict__ tw) {
+    static_assert(G >= 4 && G <= 32, "exchange network: 4- to 32-lane groups");
+    constexpr int RR = xregs(R), H = RR / 2;
     int st = (G / 2) * R;
 #pragma unroll
     for (int h = 1; h <= G / 2; h <<= 1) {
@@ -229,7 +230,7 @@ __device__ __forceinline__ void wfft_dit_x(V (&v)[R], int g, const V* __restrict
         }
         st >>= 1;
     }
-    rotate_halves<R>(v, (g & (G / 2)) != 0);
+    rotate_halves<RR>(v, (g & (G / 2)) != 0);
     if (g != 0) {
 #pragma unroll
         for (int k1 = 1; k1 < R; ++k1) {
@@ -238,10 +239,11 @@ __device__ __forceinline__ void wfft_dit_x(V (&v)[R], int g, const V* __restrict
             v[k1] = cmul(v[k1], w);
         }
     }
-    dft_reg<R, SIGN>(v);
+    dft_first<R, SIGN>(v);
 }
 
-// physical pair index of register k of lane g after a product-row c2r (the slot layout)
+// physical pair index of register k of lane g after an FP32 product-row c2r (the slot layout of
+// the lane-pair network for odd R)
 template <int R>
 __device__ __forceinline__ int nl_pair(int g, int k) {
     if constexpr (R % 2 == 0) return xslot<R, 32>(g, k);
@@ -307,7 +309,7 @@ struct alignas(64) YTmaMaps {
 // the transform's cross-lane stages unroll and their twiddle loads are issued up front;
 // 64 registers (4 blocks per SM) fit the unrolled FP64 form without spills
 template <int R, bool INV, int GC = 0, bool TMA = false>
-__global__ void __launch_bounds__(256, 4) k_ywarp(YInvJobList ij, YFwdJobList fj, YPassArgs a, int nch,
+__global__ void __launch_bounds__(256, R <= 8 ? 4 : (R <= 9 ? 3 : 2)) k_ywarp(YInvJobList ij, YFwdJobList fj, YPassArgs a, int nch,
                                                   const __grid_constant__ YTmaMaps tm) {
     extern __shared__ __align__(1024) unsigned char ysm_raw[];
     // the TMA's 128-byte swizzle wants 1024-byte aligned destinations
@@ -418,7 +420,8 @@ __global__ void __launch_bounds__(256, 4) k_ywarp(YInvJobList ij, YFwdJobList fj
             const int L = L0 + q;
             const bool act = L < WKC;
             const int Lc = act ? L : 0;
-            double2 v[R];
+            constexpr bool XN = GC >= 4 && R > 1;  // exchange network: register k1 holds output xslot(g, k1)
+            double2 v[XN ? xregs(R) : R];
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const int n = g + G * r;
@@ -436,12 +439,14 @@ __global__ void __launch_bounds__(256, 4) k_ywarp(YInvJobList ij, YFwdJobList fj
                 }
                 v[r] = x;
             }
-            if constexpr (GC == 16 && R % 2 == 0) {
-                // exchange network: register k1 holds output xslot(g, k1)
-                wfft_x<R, INV ? +1 : -1, 16>(v, g, a.plan.tw);
+            if constexpr (XN) {
+                wfft_x<R, INV ? +1 : -1, GC>(v, g, a.plan.tw);
                 if (act) {
 #pragma unroll
-                    for (int k1 = 0; k1 < R; ++k1) T[IX(xslot<R, 16>(g, k1), L)] = v[k1];
+                    for (int k1 = 0; k1 < xregs(R); ++k1) {
+                        const int n = xslot<R, GC>(g, k1);
+                        if (R % 2 == 0 || n >= 0) T[IX(n, L)] = v[k1];
+                    }
                 }
             } else {
                 wfft<R, INV ? +1 : -1>(v, G, g, a.plan.tw);
@@ -540,9 +545,10 @@ __global__ void __launch_bounds__(256, 4) k_ywarp(YInvJobList ij, YFwdJobList fj
 template <class V>
 __device__ __forceinline__ int xsw(int n) { return sizeof(V) == 16 ? (n ^ ((n >> 3) & 7)) : n; }
 
-template <int R, bool XN, class V>
+// XG: the lane-group width of an exchange network, 0: the lane-pair network
+template <int R, int XG, class V>
 __device__ __forceinline__ void row_c2r_regs(const V* X, int N, int G, int g, const V* __restrict__ twr,
-                                             const V* __restrict__ tw, V (&v)[R]) {
+                                             const V* __restrict__ tw, V (&v)[XG ? xregs(R) : R]) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int n = g + G * r;
@@ -552,7 +558,7 @@ __device__ __forceinline__ void row_c2r_regs(const V* X, int N, int G, int g, co
         const V o = cmul(csub(xa, xb), cconj(__ldg(&twr[n])));
         v[r] = CT<V>::make(e.x - o.y, e.y + o.x);
     }
-    if constexpr (XN) wfft_x<R, +1, 32>(v, g, tw);
+    if constexpr (XG != 0) wfft_x<R, +1, XG>(v, g, tw);
     else wfft<R, +1>(v, G, g, tw);
 }
 
@@ -620,18 +626,21 @@ __global__ void __launch_bounds__(256) k_row_c2r_w(RowJobList jobs, RowArgs a) {
             X[xsw<V>(k)] = v;
         }
         __syncwarp();
-        V v[R];
-        constexpr bool XN = (GC == 32 && R % 2 == 0);  // exchange network
-        row_c2r_regs<R, XN>(X, N, G, g, twr, tw, v);
+        // exchange network (odd R in FP64)
+        constexpr int XG = (GC != 0 && R > 1 && (R % 2 == 0 || sizeof(S) == 8)) ? GC : 0;
+        constexpr int RR = XG ? xregs(R) : R;
+        V v[RR];
+        row_c2r_regs<R, XG>(X, N, G, g, twr, tw, v);
         S m = (S)0;
         if (job.mean != nullptr && job.add_mean != 0.0) m = (S)(job.mean[row / a.nyl] * job.add_mean);
         const S sc = (S)job.scale;
-        if constexpr (!XN) lane_bitrev<R>(v, G, lane, g, lgg);
+        if constexpr (!XG) lane_bitrev<R>(v, G, lane, g, lgg);
         __syncwarp();
 #pragma unroll
-        for (int k1 = 0; k1 < R; ++k1) {
+        for (int k1 = 0; k1 < RR; ++k1) {
             int n = R * g + k1;
-            if constexpr (XN) n = xslot<R, 32>(g, k1);
+            if constexpr (XG != 0) n = xslot<R, XG>(g, k1);
+            if (XG != 0 && R % 2 == 1 && n < 0) continue;
             X[xsw<V>(n)] = CT<V>::make(sc * v[k1].x + m, sc * v[k1].y + m);
         }
         __syncwarp();
@@ -717,7 +726,7 @@ __global__ void __launch_bounds__(128) k_row_c2r_dyn(DynRowArgs a) {
             }
             load_row(i < 11 ? src_of(row, i + 1) : src_of(row + W, 0));
             __syncwarp();
-            row_c2r_regs<R, true>(X, N, 32, g, twr, tw, v);
+            row_c2r_regs<R, 32>(X, N, 32, g, twr, tw, v);
         };
         // a physical row from the slot layout, written in coalesced order through the buffer
         auto store = [&](double* out, const V (&v)[R]) {
@@ -850,7 +859,7 @@ __global__ void __launch_bounds__(256) k_row_r2c_w(RowJobList jobs, RowArgs a) {
     }
 }
 
-// r2c row pass for full-warp plans (G = 32, N = 32 R): one warp per row, the physical row
+// r2c row pass: one lane group of GC lanes per row (N = GC R), the physical row
 // staged in shared memory under an XOR swizzle, so that both its natural-order writes
 // (lane-contiguous) and its slot-order reads (stride R, lanes bit-reversed) are free of
 // bank conflicts; the decimation-in-time network then ends in natural order, where the
@@ -867,60 +876,69 @@ __device__ __forceinline__ int rsw_x(int n) {
     else return n ^ ((n >> 3) & 7);
 }
 
-template <int R, class V>
+template <int R, class V, int GC = 32>
 __global__ void __launch_bounds__(256) k_row_r2c_s(RowJobList jobs, RowArgs a) {
     using S = typename CT<V>::S;
-    constexpr int N = 32 * R, LS = N + 8;
+    constexpr int N = GC * R, LS = N + 8, LPW = 32 / GC;
+    // exchange network (odd R in FP64), else the lane-pair one
+    constexpr bool XN = R % 2 == 0 || (R > 1 && sizeof(S) == 8);
+    constexpr int RR = XN ? xregs(R) : R;
     extern __shared__ unsigned char rsm_raw[];
     const V* twr = sizeof(S) == 4 ? reinterpret_cast<const V*>(a.rp.twrf) : reinterpret_cast<const V*>(a.rp.twr);
     const V* tw = sizeof(S) == 4 ? reinterpret_cast<const V*>(a.rp.half.twf) : reinterpret_cast<const V*>(a.rp.half.tw);
-    const int g = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    V* Z = reinterpret_cast<V*>(rsm_raw) + warp * LS;
-    const int K = a.kxc, mb = R * brev(g, 5);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int q = lane / GC, g = lane - q * GC;
+    V* Z = reinterpret_cast<V*>(rsm_raw) + (warp * LPW + q) * LS;
+    const int K = a.kxc, mb = R * brev(g, ilog2c(GC));
     const int nrows = a.nyl * a.nzp;
     const int nunits = jobs.n * nrows;
     const int gw = blockIdx.x * 8 + warp, TW = gridDim.x * 8;
-    const int src = (32 - g) & 31;
+    const int src = (lane & ~(GC - 1)) | ((GC - g) & (GC - 1));
     const S h = (S)0.5;
-    auto load_unit = [&](int u, V (&v_)[R]) {
+    auto load_unit = [&](int u0_, V (&v_)[R]) {
+        const int u = (LPW == 1 || u0_ + q < nunits) ? u0_ + q : nunits - 1;
         const int jbb = u / nrows, roww = u - jbb * nrows;
         const V* in = reinterpret_cast<const V*>(reinterpret_cast<const S*>(jobs.j[jbb].yin) + (long long)roww * a.row_pitch);
 #pragma unroll
-        for (int r = 0; r < R; ++r) v_[r] = in[g + 32 * r];
+        for (int r = 0; r < R; ++r) v_[r] = in[g + GC * r];
     };
     V nx_v[R];
-    if (gw < nunits) load_unit(gw, nx_v);
-    (void)N;
-    for (int u = gw; u < nunits; u += TW) {
+    if (gw * LPW < nunits) load_unit(gw * LPW, nx_v);
+    for (int u0 = gw * LPW; u0 < nunits; u0 += TW * LPW) {
+        const bool act = LPW == 1 || u0 + q < nunits;  // a group past the last row repeats it, unstored
+        const int u = act ? u0 + q : nunits - 1;
         const int jb = u / nrows, row = u - jb * nrows;
         const RowIO job = jobs.j[jb];
-        V v[R];
+        V v[RR];
         if (job.lam != nullptr) {  // fringe forcing lambda(x) (m - q) on the fly
             const S m = (job.mean != nullptr && job.add_mean != 0.0) ? (S)(job.mean[row / a.nyl] * job.add_mean) : (S)0;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                const int x = 2 * (g + 32 * r);
+                const int x = 2 * (g + GC * r);
                 const S l0 = (S)job.lam[x], l1 = (S)job.lam[x + 1];
                 nx_v[r] = CT<V>::make(l0 * (m - nx_v[r].x), l1 * (m - nx_v[r].y));
             }
         }
 #pragma unroll
-        for (int r = 0; r < R; ++r) Z[rsw_x<R>(g + 32 * r)] = nx_v[r];
-        if (u + TW < nunits) load_unit(u + TW, nx_v);
+        for (int r = 0; r < R; ++r) Z[rsw_x<R>(g + GC * r)] = nx_v[r];
+        if (u0 + TW * LPW < nunits) load_unit(u0 + TW * LPW, nx_v);
         __syncwarp();
-        if constexpr (R % 2 == 0) {
+        if constexpr (XN) {
             // the exchange network's input layout: register k1 holds z[xslot(g, k1)]
 #pragma unroll
-            for (int k1 = 0; k1 < R; ++k1) v[k1] = Z[rsw_x<R>(xslot<R, 32>(g, k1))];
+            for (int k1 = 0; k1 < RR; ++k1) {
+                const int n = xslot<R, GC>(g, k1);
+                v[k1] = Z[rsw_x<R>((R % 2 == 1 && n < 0) ? 0 : n)];
+            }
         } else {
 #pragma unroll
             for (int k1 = 0; k1 < R; ++k1) v[k1] = Z[rsw_x<R>(k1 + mb)];
         }
         __syncwarp();  // the row buffer is free for the next row
-        if constexpr (R % 2 == 0) wfft_dit_x<R, -1, 32>(v, g, tw);
-        else wfft_dit<R, -1>(v, 32, g, tw);
-        // natural order: lane g register rr holds Z[g + 32 rr]; Z[N-k] for k = g + 32 rr is
-        // lane (32-g) register R-1-rr (g > 0), or lane 0 register R-rr (g = 0, rr > 0)
+        if constexpr (XN) wfft_dit_x<R, -1, GC>(v, g, tw);
+        else wfft_dit<R, -1>(v, GC, g, tw);
+        // natural order: lane g register rr holds Z[g + GC rr]; Z[N-k] for k = g + GC rr is
+        // lane (GC-g) register R-1-rr (g > 0), or lane 0 register R-rr (g = 0, rr > 0)
         V* yrow = reinterpret_cast<V*>(reinterpret_cast<S*>(job.out) + (long long)row * 2 * K);
 #pragma unroll
         for (int rr = 0; rr < R; ++rr) {
@@ -928,8 +946,8 @@ __global__ void __launch_bounds__(256) k_row_r2c_s(RowJobList jobs, RowArgs a) {
             zb.x = __shfl_sync(0xffffffffu, v[R - 1 - rr].x, src);
             zb.y = __shfl_sync(0xffffffffu, v[R - 1 - rr].y, src);
             if (g == 0) zb = v[rr == 0 ? 0 : R - rr];
-            const int k = g + 32 * rr;
-            if (k < K) {
+            const int k = g + GC * rr;
+            if (act && k < K) {
                 const V za = v[rr];
                 zb = cconj(zb);
                 const V e = CT<V>::make(h * (za.x + zb.x), h * (za.y + zb.y));
@@ -1036,7 +1054,10 @@ __global__ void __launch_bounds__(256, 2) k_row_nl_w(NlRowArgs a) {
     const int lpw = 32 / G, q = lane / G, g = lane - q * G;
     double2* Stg[2] = {smem, smem + 9 * K};   // staged rows: U0..2, DY0..2, DZ0..2
     double2* P = smem + 18 * K;               // 12 physical rows of N complex (2N reals)
-    double2* W = P + 12 * N + (warp * lpw + q) * (N + 1);
+    // r2c lines: one per field when a pass over the lane groups covers the nine (G < 32), else
+    // one per group
+    const int wl = 8 * lpw >= 9 ? min(warp * lpw + q, 8) : warp * lpw + q;
+    double2* W = P + 12 * N + wl * (N + 1);
     const int nitems = r.nyl * r.nzp;
     auto issue = [&](int row, double2* S) {
         for (int idx = tid; idx < 9 * K; idx += 256) {
@@ -1143,8 +1164,10 @@ __global__ void __launch_bounds__(256, 2) k_row_nl_w(NlRowArgs a) {
             for (int k1 = 0; k1 < R; ++k1) v[k1] = P[fc * N + k1 * G + g];
             wfft_dit<R, -1>(v, G, g, r.rp.half.tw);
             // natural order: lane g register rr holds Z[g + G*rr]
+            if (act) {
 #pragma unroll
-            for (int rr = 0; rr < R; ++rr) W[g + G * rr] = v[rr];
+                for (int rr = 0; rr < R; ++rr) W[g + G * rr] = v[rr];
+            }
             __syncwarp();
             if (act) {
                 double* dst = (fc < 3) ? a.N[fc] : a.H[fc - 3];
@@ -1159,27 +1182,27 @@ __global__ void __launch_bounds__(256, 2) k_row_nl_w(NlRowArgs a) {
     }
 }
 
-// Register-resident variant for rows of N = 32*R complex (G = 32): each warp owns a whole
+// Register-resident variant for rows of N = G*R complex: each group of G lanes owns a whole
 // (z, y) row.  Its lanes read the 9 input rows straight from global memory (coalesced),
 // and the 12 c2r, the products and the 9 r2c all stay in registers: every c2r leaves the
-// same slot layout (lane g, register k1 -> physical pair m = k1 + R*bitrev(g)), so the
-// products are lane-local, and the r2c (decimation in time from that layout) ends in
-// natural order, where the pair Z[k], Z[N-k] of the real-to-complex split is one shuffle
-// apart.  No shared memory and no block barrier.
-#ifndef NLR_MINB
-#define NLR_MINB 3
-#endif
-#ifndef NLR_SEL
-#define NLR_SEL 1
-#endif
-template <int R, class S, class V, bool SEL = (sizeof(S) == 8 && NLR_SEL)>
-__device__ __forceinline__ void nl_c2r_r(const S* __restrict__ src, bool ikx, int K, int N, int g,
+// same slot layout, so the products are lane-local, and the r2c (decimation in time from that
+// layout) ends in natural order, where the pair Z[k], Z[N-k] of the real-to-complex split is one
+// shuffle apart.  No block barrier; bound by FP64 and shuffle issue at 12 warps per SM (R up to
+// 8; 8 warps above).  Measured: 384 modes (R = 12, 96 x 129 rows) 2488 us as radix-4 stages in
+// shared memory with block barriers, 904 us here; 144 modes (R = 9 on 16 lanes, 72 x 81 rows)
+// 221 -> 169 us; 288 modes (R = 9, 36 x 64 rows) 378 -> 120 us.
+// registers of a product row's transform: FP64 rows use the exchange network, with a dummy
+// register for odd R; FP32 rows of odd R the lane-pair network
+template <int R, class V>
+constexpr int NLRR = sizeof(V) == 16 ? xregs(R) : R;
+template <int R, int GC, class S, class V>
+__device__ __forceinline__ void nl_c2r_r(const S* __restrict__ src, bool ikx, int K, int N, int G, int g,
                                          const double* __restrict__ wavx, const V* __restrict__ twr,
-                                         const V* __restrict__ tw, V (&v)[R]) {
+                                         const V* __restrict__ tw, V (&v)[NLRR<R, V>]) {
     const V zero = CT<V>::make((S)0, (S)0);
 #pragma unroll
     for (int rr = 0; rr < R; ++rr) {
-        const int n = g + 32 * rr;
+        const int n = g + G * rr;
         V xa = zero, xb = zero;
         if (n < K) xa = __ldg(reinterpret_cast<const V*>(src) + n);
         if (N - n < K) xb = __ldg(reinterpret_cast<const V*>(src) + (N - n));
@@ -1195,19 +1218,19 @@ __device__ __forceinline__ void nl_c2r_r(const S* __restrict__ src, bool ikx, in
         const V o = cmul(csub(xa, xb), cconj(__ldg(&twr[n])));
         v[rr] = CT<V>::make(e.x - o.y, e.y + o.x);
     }
-    if constexpr (R % 2 == 0) wfft_x<R, +1, 32>(v, g, tw);
-    else wfft<R, +1, SEL>(v, 32, g, tw);
+    if constexpr (NLRR<R, V> % 2 == 0) wfft_x<R, +1, GC>(v, g, tw);
+    else wfft<R, +1>(v, G, g, tw);
 }
 
 // r2c of a slot-layout row; writes the K stored modes of the row at dst
-template <int R, class S, class V, bool SEL = (sizeof(S) == 8 && NLR_SEL)>
-__device__ __forceinline__ void nl_r2c_r(V (&v)[R], S* __restrict__ dst, int K, int g, const V* __restrict__ twr,
+template <int R, int GC, class S, class V>
+__device__ __forceinline__ void nl_r2c_r(V (&v)[NLRR<R, V>], S* __restrict__ dst, int K, int G, int lane, int g, bool act, const V* __restrict__ twr,
                                          const V* __restrict__ tw) {
-    if constexpr (R % 2 == 0) wfft_dit_x<R, -1, 32>(v, g, tw);
-    else wfft_dit<R, -1, SEL>(v, 32, g, tw);
-    // natural order: lane g register rr holds Z[g + 32 rr]; Z[N-k] for k = g + 32 rr is
-    // lane (32-g) register R-1-rr (g > 0), or lane 0 register R-rr (g = 0, rr > 0)
-    const int src = (32 - g) & 31;
+    if constexpr (NLRR<R, V> % 2 == 0) wfft_dit_x<R, -1, GC>(v, g, tw);
+    else wfft_dit<R, -1>(v, G, g, tw);
+    // natural order: lane g register rr holds Z[g + G rr]; Z[N-k] for k = g + G rr is
+    // lane (G-g) register R-1-rr (g > 0), or lane 0 register R-rr (g = 0, rr > 0)
+    const int src = (lane & ~(G - 1)) | ((G - g) & (G - 1));
     const S h = (S)0.5;
 #pragma unroll
     for (int rr = 0; rr < R; ++rr) {
@@ -1215,8 +1238,8 @@ __device__ __forceinline__ void nl_r2c_r(V (&v)[R], S* __restrict__ dst, int K, 
         zb.x = __shfl_sync(0xffffffffu, v[R - 1 - rr].x, src);
         zb.y = __shfl_sync(0xffffffffu, v[R - 1 - rr].y, src);
         if (g == 0) zb = v[rr == 0 ? 0 : R - rr];
-        const int k = g + 32 * rr;
-        if (32 * rr < K && k < K) {
+        const int k = g + G * rr;
+        if (act && G * rr < K && k < K) {
             const V za = v[rr];
             zb = cconj(zb);
             const V e = CT<V>::make(h * (za.x + zb.x), h * (za.y + zb.y));
@@ -1227,23 +1250,30 @@ __device__ __forceinline__ void nl_r2c_r(V (&v)[R], S* __restrict__ dst, int K, 
     }
 }
 
+// blocks of 4 warps per SM that the register budget of k_row_nl_r is held to (shared memory:
+// 8 KB R each)
+__host__ __device__ constexpr int nl_r_blocks(int R) { return R <= 2 ? 5 : (R <= 8 ? 3 : 2); }
+
 // shared memory of k_row_nl_r: per warp, the three velocity rows and the convective sum
 template <int R>
-constexpr size_t nl_r_smem() { return (size_t)4 * 4 * R * 32 * sizeof(double2); }
+constexpr size_t nl_r_smem() { return (size_t)4 * 4 * xregs(R) * 32 * sizeof(double2); }
 
-template <int R>
-__global__ void __launch_bounds__(128, (R <= 6 ? NLR_MINB : 3)) k_row_nl_r(NlRowArgs a) {
+template <int R, int GC>
+__global__ void __launch_bounds__(128, nl_r_blocks(xregs(R))) k_row_nl_r(NlRowArgs a) {
     const RowArgs& r = a.r;
-    const int N = 32 * R, K = r.kxc;
-    const int g = threadIdx.x & 31;
+    constexpr int G = GC, N = G * R, RR = xregs(R), lpw = 32 / G;
+    const int K = r.kxc;
+    const int lane = threadIdx.x & 31, q = lane / G, g = lane - q * G;
     const int nitems = r.nyl * r.nzp;
-    const int W = gridDim.x * (blockDim.x >> 5);
+    const int W = gridDim.x * (blockDim.x >> 5) * lpw;
     // the physical velocity rows of this warp's row, lane-private slots [l][k1][lane]: kept
     // in shared memory rather than registers, so that more warps fit per SM
     extern __shared__ double2 nl_r_sm[];
-    double2* us = nl_r_sm + (threadIdx.x >> 5) * (4 * R * 32);
-    auto U = [&](int l, int k1) -> double2& { return us[(l * R + k1) * 32 + g]; };
-    for (int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < nitems; row += W) {
+    double2* us = nl_r_sm + (threadIdx.x >> 5) * (4 * RR * 32);
+    auto U = [&](int l, int k1) -> double2& { return us[(l * RR + k1) * 32 + lane]; };
+    for (int row0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * lpw; row0 < nitems; row0 += W) {
+        const bool act = row0 + q < nitems;  // a group past the last row repeats it, unstored
+        const int row = act ? row0 + q : nitems - 1;
         const int z = row / r.nyl;
         const long long off = (long long)row * 2 * K;
         const double ub = a.ubar[z], ubp = a.ubarp[z];
@@ -1257,18 +1287,18 @@ __global__ void __launch_bounds__(128, (R <= 6 ? NLR_MINB : 3)) k_row_nl_r(NlRow
 #pragma unroll 1
         for (int op = 0; op < 21; ++op) {
             const int cl = (op - 9) >> 2, ct = (op - 9) & 3;  // component and step of ops 9..20
-            double2 v[R];
+            double2 v[RR];
             if (op < 3 || (op >= 9 && ct < 3)) {
                 const double* src = (op < 3) ? a.U[op] : (ct == 0 ? a.U[cl] : (ct == 1 ? a.DY[cl] : a.DZ[cl]));
-                nl_c2r_r<R>(src + off, op >= 9 && ct == 0, K, N, g, r.wavx, r.rp.twr, r.rp.half.tw, v);
+                nl_c2r_r<R, GC>(src + off, op >= 9 && ct == 0, K, N, G, g, r.wavx, r.rp.twr, r.rp.half.tw, v);
                 if (op < 3) {
                     const double add = (op == 0) ? ub : 0.0;
 #pragma unroll
-                    for (int k1 = 0; k1 < R; ++k1) U(op, k1) = make_double2(v[k1].x + add, v[k1].y + add);
+                    for (int k1 = 0; k1 < RR; ++k1) U(op, k1) = make_double2(v[k1].x + add, v[k1].y + add);
                 } else {
                     const double dzb = (ct == 2 && cl == 0) ? ubp : 0.0;
 #pragma unroll
-                    for (int k1 = 0; k1 < R; ++k1) {
+                    for (int k1 = 0; k1 < RR; ++k1) {
                         const double2 um = U(ct, k1);
                         const double2 c = (ct == 0) ? make_double2(0.0, 0.0) : U(3, k1);
                         U(3, k1) = make_double2(c.x - 0.5 * (um.x * (v[k1].x + dzb)),
@@ -1282,7 +1312,7 @@ __global__ void __launch_bounds__(128, (R <= 6 ? NLR_MINB : 3)) k_row_nl_r(NlRow
                     const int l = (p < 3) ? 0 : (p < 5 ? 1 : 2);
                     const int m = (p < 3) ? p : (p < 5 ? p - 2 : 2);
 #pragma unroll
-                    for (int k1 = 0; k1 < R; ++k1) {
+                    for (int k1 = 0; k1 < RR; ++k1) {
                         const double2 ul = U(l, k1), um = U(m, k1);
                         v[k1] = make_double2(0.5 * (ul.x * um.x), 0.5 * (ul.y * um.y));
                     }
@@ -1290,10 +1320,10 @@ __global__ void __launch_bounds__(128, (R <= 6 ? NLR_MINB : 3)) k_row_nl_r(NlRow
                 } else {
                     const double ut = (cl == 0) ? ub : 0.0;
 #pragma unroll
-                    for (int k1 = 0; k1 < R; ++k1) {
+                    for (int k1 = 0; k1 < RR; ++k1) {
                         double2 c = U(3, k1);
                         if (a.lamx != nullptr) {
-                            const int x = 2 * nl_pair<R>(g, k1);  // physical x of the pair in register k1
+                            const int x = 2 * max(xslot<R, GC>(g, k1), 0);  // physical x of the pair in register k1
                             const double lx0 = __ldg(&a.lamx[x]), lx1 = __ldg(&a.lamx[x + 1]);
                             const double2 ul = U(cl, k1);
                             c.x = c.x + lx0 * (ut - ul.x);
@@ -1303,7 +1333,7 @@ __global__ void __launch_bounds__(128, (R <= 6 ? NLR_MINB : 3)) k_row_nl_r(NlRow
                     }
                     dst = a.N[cl];
                 }
-                nl_r2c_r<R>(v, dst + off, K, g, r.rp.twr, r.rp.half.tw);
+                nl_r2c_r<R, GC>(v, dst + off, K, G, lane, g, act, r.rp.twr, r.rp.half.tw);
             }
         }
     }
@@ -1534,7 +1564,7 @@ __global__ void __launch_bounds__(128, NLF_MINB) k_row_nl_f(NlRowArgs a) {
 #pragma unroll 1
         for (int l = 0; l < 3; ++l) {
             float2 t[R];
-            nl_c2r_r<R>(F(a.U[l]) + off, false, K, N, g, r.wavx, r.rp.twrf, r.rp.half.twf, t);
+            nl_c2r_r<R, 32>(F(a.U[l]) + off, false, K, N, 32, g, r.wavx, r.rp.twrf, r.rp.half.twf, t);
 #pragma unroll
             for (int k1 = 0; k1 < R; ++k1) U(l, k1) = t[k1];
         }
@@ -1556,7 +1586,7 @@ __global__ void __launch_bounds__(128, NLF_MINB) k_row_nl_f(NlRowArgs a) {
                     f[k1] = make_float2(0.5f * (ul.x * um.x), 0.5f * (ul.y * um.y));
                 }
             }
-            nl_r2c_r<R>(f, reinterpret_cast<float*>(a.H[p]) + off, K, g, r.rp.twrf, r.rp.half.twf);
+            nl_r2c_r<R, 32>(f, reinterpret_cast<float*>(a.H[p]) + off, K, 32, g, g, true, r.rp.twrf, r.rp.half.twf);
         }
 #pragma unroll 1
         for (int l = 0; l < 3; ++l) {
@@ -1565,7 +1595,7 @@ __global__ void __launch_bounds__(128, NLF_MINB) k_row_nl_f(NlRowArgs a) {
 #pragma unroll 1
             for (int t = 0; t < 3; ++t) {
                 const double* src = (t == 0) ? a.U[l] : (t == 1 ? a.DY[l] : a.DZ[l]);
-                nl_c2r_r<R>(F(src) + off, t == 0, K, N, g, r.wavx, r.rp.twrf, r.rp.half.twf, d);
+                nl_c2r_r<R, 32>(F(src) + off, t == 0, K, N, 32, g, r.wavx, r.rp.twrf, r.rp.half.twf, d);
                 const float dzb = (t == 2 && l == 0) ? ubp : 0.f;
                 const float um0 = (t == 0) ? ub : 0.f;  // u' carries the mean ubar only in u_1
 #pragma unroll
@@ -1588,7 +1618,7 @@ __global__ void __launch_bounds__(128, NLF_MINB) k_row_nl_f(NlRowArgs a) {
                 }
                 d[k1] = c;
             }
-            nl_r2c_r<R>(d, reinterpret_cast<float*>(a.N[l]) + off, K, g, r.rp.twrf, r.rp.half.twf);
+            nl_r2c_r<R, 32>(d, reinterpret_cast<float*>(a.N[l]) + off, K, 32, g, g, true, r.rp.twrf, r.rp.half.twf);
         }
     }
 }
@@ -1603,7 +1633,7 @@ template <int R, bool INV>
 void ylaunch(const YInvJobList& ij, const YFwdJobList& fj, const YPassArgs& a, cudaStream_t s) {
     const int nch = (a.kxc + WKC - 1) / WKC;
     const int nitems = (INV ? ij.n : fj.n) * a.nzp * nch;
-    if (a.f32) {
+    if constexpr (R <= 4 || R == 6 || R == 8) if (a.f32) {
         const size_t smf = (size_t)2 * a.nyl * WKC * sizeof(double2);
         lsb::note_launch();
         if (a.plan.g == 16) k_ywarp_f<R, INV, 16><<<persistent_grid_w(k_ywarp_f<R, INV, 16>, smf, nitems), 256, smf, s>>>(ij, fj, a, nch);
@@ -1632,13 +1662,21 @@ void ylaunch(const YInvJobList& ij, const YFwdJobList& fj, const YPassArgs& a, c
                               : (size_t)2 * a.nyl * (WKC + 1) * sizeof(double2);
     lsb::note_launch();
     auto go = [&](auto kern) { kern<<<persistent_grid_w(kern, sm, nitems), 256, sm, s>>>(ij, fj, a, nch, tm); };
-    if (use_tma) {
-        if (a.plan.g == 16) go(k_ywarp<R, INV, 16, true>);
-        else go(k_ywarp<R, INV, 0, true>);
+    if (a.plan.g == 16) {
+        use_tma ? go(k_ywarp<R, INV, 16, true>) : go(k_ywarp<R, INV, 16>);
         return;
     }
-    if (a.plan.g == 16) go(k_ywarp<R, INV, 16>);
-    else go(k_ywarp<R, INV>);
+    if constexpr (R % 2 == 1 && R > 1) {  // (groups of 8 and 4 lanes come with an odd R)
+        if (a.plan.g == 8) {
+            use_tma ? go(k_ywarp<R, INV, 8, true>) : go(k_ywarp<R, INV, 8>);
+            return;
+        }
+        if (a.plan.g == 4 && !use_tma) {
+            go(k_ywarp<R, INV, 4>);
+            return;
+        }
+    }
+    use_tma ? go(k_ywarp<R, INV, 0, true>) : go(k_ywarp<R, INV>);
 }
 
 template <bool INV>
@@ -1650,6 +1688,10 @@ bool ydispatch(const YInvJobList& ij, const YFwdJobList& fj, const YPassArgs& a,
         case 4: ylaunch<4, INV>(ij, fj, a, s); return true;
         case 6: ylaunch<6, INV>(ij, fj, a, s); return true;
         case 8: ylaunch<8, INV>(ij, fj, a, s); return true;
+        case 5: ylaunch<5, INV>(ij, fj, a, s); return true;
+        case 7: ylaunch<7, INV>(ij, fj, a, s); return true;
+        case 9: ylaunch<9, INV>(ij, fj, a, s); return true;
+        case 15: ylaunch<15, INV>(ij, fj, a, s); return true;
         default: return false;
     }
 }
@@ -1660,28 +1702,37 @@ void rowlaunch_t(const RowJobList& jobs, const RowArgs& a, cudaStream_t s, bool 
     const size_t sm = (size_t)8 * 32 * (N + 8) * sizeof(V) / a.rp.half.g;  // row stride N + 8 (swizzle)
     const long long units = (long long)jobs.n * a.nyl * a.nzp;
     const long long blocks = (units + 8 * 32 / a.rp.half.g - 1) / (8 * 32 / a.rp.half.g);
-    const bool g32 = a.rp.half.g == 32;
-    if (!c2r && g32 && N == 32 * R) {
-        const size_t ss = (size_t)8 * (N + 8) * sizeof(V);
-        const long long b32 = (units + 7) / 8;
+    const int G = a.rp.half.g;
+    auto go = [&](auto kern) {
         lsb::note_launch();
-        k_row_r2c_s<R, V><<<persistent_grid_w(k_row_r2c_s<R, V>, ss, b32), 256, ss, s>>>(jobs, a);
+        kern<<<persistent_grid_w(kern, sm, blocks), 256, sm, s>>>(jobs, a);
+    };
+    if (G == 32) {
+        c2r ? go(k_row_c2r_w<R, V, 32>) : go(k_row_r2c_s<R, V, 32>);
         return;
     }
-    lsb::note_launch();
-    if (c2r) {
-        if (g32) k_row_c2r_w<R, V, 32><<<persistent_grid_w(k_row_c2r_w<R, V, 32>, sm, blocks), 256, sm, s>>>(jobs, a);
-        else k_row_c2r_w<R, V><<<persistent_grid_w(k_row_c2r_w<R, V>, sm, blocks), 256, sm, s>>>(jobs, a);
-    } else {
-        if (g32) k_row_r2c_w<R, V, 32><<<persistent_grid_w(k_row_r2c_w<R, V, 32>, sm, blocks), 256, sm, s>>>(jobs, a);
-        else k_row_r2c_w<R, V><<<persistent_grid_w(k_row_r2c_w<R, V>, sm, blocks), 256, sm, s>>>(jobs, a);
+    if constexpr (R % 2 == 1 && R > 1 && sizeof(V) == 16) {  // (narrower groups come with an odd R)
+        if (G == 16) {
+            c2r ? go(k_row_c2r_w<R, V, 16>) : go(k_row_r2c_s<R, V, 16>);
+            return;
+        }
+        if (G == 8) {
+            c2r ? go(k_row_c2r_w<R, V, 8>) : go(k_row_r2c_s<R, V, 8>);
+            return;
+        }
     }
+    c2r ? go(k_row_c2r_w<R, V>) : go(k_row_r2c_w<R, V>);
 }
 
 template <int R>
 void rowlaunch(const RowJobList& jobs, const RowArgs& a, cudaStream_t s, bool c2r) {
-    if (a.f32) rowlaunch_t<R, float2>(jobs, a, s, c2r);
-    else rowlaunch_t<R, double2>(jobs, a, s, c2r);
+    if constexpr (R <= 4 || R == 6 || R == 8) {
+        if (a.f32) {
+            rowlaunch_t<R, float2>(jobs, a, s, c2r);
+            return;
+        }
+    }
+    rowlaunch_t<R, double2>(jobs, a, s, c2r);
 }
 
 bool rowdispatch(const RowJobList& jobs, const RowArgs& a, cudaStream_t s, bool c2r) {
@@ -1692,6 +1743,11 @@ bool rowdispatch(const RowJobList& jobs, const RowArgs& a, cudaStream_t s, bool 
         case 4: rowlaunch<4>(jobs, a, s, c2r); return true;
         case 6: rowlaunch<6>(jobs, a, s, c2r); return true;
         case 8: rowlaunch<8>(jobs, a, s, c2r); return true;
+        case 5: rowlaunch<5>(jobs, a, s, c2r); return true;
+        case 7: rowlaunch<7>(jobs, a, s, c2r); return true;
+        case 9: rowlaunch<9>(jobs, a, s, c2r); return true;
+        case 12: rowlaunch<12>(jobs, a, s, c2r); return true;
+        case 15: rowlaunch<15>(jobs, a, s, c2r); return true;
         default: return false;
     }
 }
@@ -1700,7 +1756,7 @@ template <int R>
 void nllaunch(const NlRowArgs& a, cudaStream_t s) {
     const int N = a.r.nxl / 2;
     const int nitems = a.r.nyl * a.r.nzp;
-    if (a.r.f32) {
+    if constexpr (R <= 4 || R == 6 || R == 8) if (a.r.f32) {
         if (a.r.rp.half.g != 32) throw std::runtime_error("mixed precision: x transform length has no full-warp plan");
         constexpr size_t sm = nl_f_smem<R>();
         if (!allow_smem((const void*)k_row_nl_f<R>, sm))
@@ -1711,42 +1767,76 @@ void nllaunch(const NlRowArgs& a, cudaStream_t s) {
         { lsb::note_launch(); k_row_nl_f<R><<<(int)blocks, 128, sm, s>>>(a); }
         return;
     }
-    if (a.r.rp.half.g == 32) {
-        constexpr size_t sm = nl_r_smem<R>();
-        if (!allow_smem((const void*)k_row_nl_r<R>, sm))
+    const int G = a.r.rp.half.g;
+    auto rows = [&](auto kern, int lanes, size_t sm) {
+        if (!allow_smem((const void*)kern, sm))
             throw std::runtime_error("product rows: shared memory of the register plan refused");
-        const int occ = resident_blocks((const void*)k_row_nl_r<R>, 128, sm);
-        long long blocks = (long long)occ * sm_count(), need = (nitems + 3) / 4;
+        const int occ = resident_blocks((const void*)kern, 128, sm);
+        const long long units = (nitems + 32 / lanes - 1) / (32 / lanes);  // warps' rows
+        long long blocks = (long long)occ * sm_count(), need = (units + 3) / 4;
         if (blocks > need) blocks = need > 0 ? need : 1;
-        { lsb::note_launch(); k_row_nl_r<R><<<(int)blocks, 128, sm, s>>>(a); }
-        return;
+        lsb::note_launch();
+        kern<<<(int)blocks, 128, sm, s>>>(a);
+    };
+    // Register rows: even R with the exchange network on full warps, odd R with its dummy
+    // register on the plan's groups.  R = 1 and full warps of R = 3 take half the lanes with twice
+    // the registers, which wastes none: 96 modes, 48 x 65 rows 58.5 us in the lane-pair network,
+    // 55.7 with the dummy, 45.1 on 16 lanes (48 modes, 24 x 65 rows the other way round: 27.8 on 8
+    // lanes, 21.7 on 16 with the dummy: too few warps).
+    if constexpr (R % 2 == 0) {
+        if (G == 32) {
+            rows(k_row_nl_r<R, 32>, 32, nl_r_smem<R>());
+            return;
+        }
+    } else if constexpr (R == 1) {
+        switch (G) {
+            case 32: rows(k_row_nl_r<2, 16>, 16, nl_r_smem<2>()); return;
+            case 16: rows(k_row_nl_r<2, 8>, 8, nl_r_smem<2>()); return;
+            case 8: rows(k_row_nl_r<2, 4>, 4, nl_r_smem<2>()); return;
+            default: break;
+        }
+    } else if constexpr (R <= 9) {
+        switch (G) {
+            case 32:
+                if constexpr (R == 3) rows(k_row_nl_r<6, 16>, 16, nl_r_smem<6>());
+                else rows(k_row_nl_r<R, 32>, 32, nl_r_smem<R>());
+                return;
+            case 16: rows(k_row_nl_r<R, 16>, 16, nl_r_smem<R>()); return;
+            case 8: rows(k_row_nl_r<R, 8>, 8, nl_r_smem<R>()); return;
+            case 4: rows(k_row_nl_r<R, 4>, 4, nl_r_smem<R>()); return;
+            default: break;
+        }
     }
+    if constexpr (R % 2 == 1) {  // (an even R always comes with full warps)
     const size_t sm =
-        ((size_t)18 * a.r.kxc + (size_t)12 * N + (size_t)8 * 32 / a.r.rp.half.g * (N + 1)) * sizeof(double2);
+        ((size_t)18 * a.r.kxc + (size_t)12 * N + (size_t)(a.r.rp.half.g < 32 ? 9 : 8) * (N + 1)) * sizeof(double2);
     { lsb::note_launch(); k_row_nl_w<R><<<persistent_grid_w(k_row_nl_w<R>, sm, nitems), 256, sm, s>>>(a); }
+    } else {
+        throw std::runtime_error("product rows: no kernel for this plan");
+    }
 }
 
 }  // namespace
 
 bool launch_yinv_warp(const YInvJobList& jobs, const YPassArgs& a, cudaStream_t s) {
-    if (a.plan.g == 0) return false;
+    if (a.plan.g == 0 || (a.f32 && a.plan.fp64_only)) return false;
     YFwdJobList none{};
     return ydispatch<true>(jobs, none, a, s);
 }
 
 bool launch_yfwd_warp(const YFwdJobList& jobs, const YPassArgs& a, cudaStream_t s) {
-    if (a.plan.g == 0) return false;
+    if (a.plan.g == 0 || (a.f32 && a.plan.fp64_only)) return false;
     YInvJobList none{};
     return ydispatch<false>(none, jobs, a, s);
 }
 
 bool launch_row_c2r_warp(const RowJobList& jobs, const RowArgs& a, cudaStream_t s) {
-    if (a.rp.half.g == 0) return false;
+    if (a.rp.half.g == 0 || (a.f32 && a.rp.half.fp64_only)) return false;
     return rowdispatch(jobs, a, s, true);
 }
 
 bool launch_row_r2c_warp(const RowJobList& jobs, const RowArgs& a, cudaStream_t s) {
-    if (a.rp.half.g == 0) return false;
+    if (a.rp.half.g == 0 || (a.f32 && a.rp.half.fp64_only)) return false;
     return rowdispatch(jobs, a, s, false);
 }
 
@@ -1809,7 +1899,7 @@ void launch_row_c2r_dyn(const DynRowArgs& a, cudaStream_t s) {
 }
 
 bool launch_row_nl_warp(const NlRowArgs& a, cudaStream_t s) {
-    if (a.r.rp.half.g == 0) return false;
+    if (a.r.rp.half.g == 0 || (a.r.f32 && a.r.rp.half.fp64_only)) return false;
     switch (a.r.rp.half.r) {
         case 1: nllaunch<1>(a, s); return true;
         case 2: nllaunch<2>(a, s); return true;
@@ -1817,6 +1907,11 @@ bool launch_row_nl_warp(const NlRowArgs& a, cudaStream_t s) {
         case 4: nllaunch<4>(a, s); return true;
         case 6: nllaunch<6>(a, s); return true;
         case 8: nllaunch<8>(a, s); return true;
+        case 5: nllaunch<5>(a, s); return true;
+        case 7: nllaunch<7>(a, s); return true;
+        case 9: nllaunch<9>(a, s); return true;
+        case 12: nllaunch<12>(a, s); return true;
+        case 15: nllaunch<15>(a, s); return true;
         default: return false;
     }
 }

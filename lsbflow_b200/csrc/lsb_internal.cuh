@@ -55,6 +55,7 @@ struct FftPlan {
     const float2* twf = nullptr;   // the same in FP32
     int n1 = 0, n2 = 0;            // register two-pass split n = n1*n2 (n1 = 0: Stockham stages)
     int g = 0, r = 0, lgg = 0;     // warp-group split n = g*r (g lanes, r registers; g = 0: none)
+    bool fp64_only = false;        // the split's r is one that only the FP64 kernels have
     int ls = 0;                    // shared-memory line stride (complex) a kernel must use
 };
 

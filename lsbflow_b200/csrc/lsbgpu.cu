@@ -118,13 +118,19 @@ void make_plan(lsb_handle* h, int n, FftPlan& P, int max_g = 32) {
     if (ls % 2 == 0) ++ls;
     P.ls = ls;
     // warp-group split: g = the largest power of two <= max_g dividing n, widened (up to 32)
-    // until r = n / g is in {1,2,3,4,6,8}
+    // until r = n / g is in {1,2,3,4,6,8}; lengths without one take r in {5,7,9,12,15} in the
+    // same way, in FP64 only
     P.g = P.r = P.lgg = 0;
-    {
+    for (const bool ext : {false, true}) {
         int gg = 1;
         while (gg < max_g && n % (gg * 2) == 0) gg *= 2;
-        auto ok = [](int r) { return r == 1 || r == 2 || r == 3 || r == 4 || r == 6 || r == 8; };
+        auto ok = [ext](int r) {
+            return ext ? r == 5 || r == 7 || r == 9 || r == 12 || r == 15
+                       : r == 1 || r == 2 || r == 3 || r == 4 || r == 6 || r == 8;
+        };
         while (!ok(n / gg) && gg < 32 && n % (gg * 2) == 0) gg *= 2;
+        if (P.g != 0) break;
+        P.fp64_only = ext;
         const int rr = n / gg;
         if (n % gg == 0 && ok(rr)) {
             P.g = gg;
@@ -1318,8 +1324,10 @@ int lsb_create(const lsb_config* cfg, const lsb_setup* su, lsb_handle** out) {
             const bool phys = cfg->sgsflag == 1 || (dl && cfg->forcing == 1);
             // the nonlinear term's (padded) passes in FP32 where their lengths have full-warp
             // register plans, else in FP64 (the 3/2-rule x length 48 of a 64-point grid)
-            h->nl_f32 = (dl ? h->pyl : h->py).g != 0 && (dl ? h->rxl : h->rx).half.g == 32;
-            if ((!dl && !h->nl_f32) || (phys && (h->py.g == 0 || h->rx.half.g == 0)))
+            auto f32 = [](const FftPlan& p) { return p.g != 0 && !p.fp64_only; };
+            const FftPlan &yp = dl ? h->pyl : h->py, &xp = (dl ? h->rxl : h->rx).half;
+            h->nl_f32 = f32(yp) && f32(xp) && xp.g == 32;
+            if ((!dl && !h->nl_f32) || (phys && (!f32(h->py) || !f32(h->rx.half))))
                 fail(LSB_ERR_ARG, "mixed precision needs transform lengths with register plans: x/2 a multiple of "
                                   "32 (32 R, R in 1,2,3,4,6,8) and y a power of two times 1,2,3,4,6,8");
         }
