@@ -153,9 +153,10 @@ typedef struct {
                             contractions at 5, 7 and 8 */
     int filter_zchunks;  /* 3-point SGS test filter: z chunks a block column is split into,
                             1..(nzp+3)/4; 0 = the waves x planes-per-block model */
-    int y_staging;       /* FP64 spanwise passes: tiles staged by cp.async (1) or by TMA tile
-                            loads (2); 0 = the built-in choice (TMA on the padded grid,
-                            cp.async on the unpadded one) */
+    int y_staging;       /* FP64 spanwise passes in tiles (lengths without a column-per-thread
+                            pass, and the sigma model's gradients): staged by cp.async (1) or
+                            by TMA tile loads (2); 0 = the built-in choice (TMA on the padded
+                            grid, cp.async on the unpadded one) */
     int filter_staging;  /* 3-point SGS test filter: plane ring filled by cp.async (1) or by TMA
                             row loads (2, rows of a multiple of 128 bytes); 0 = the built-in
                             choice (TMA for FP64 rows, cp.async for the FP32 rows of the mixed

@@ -357,7 +357,7 @@ static int persistent_grid(K kern, size_t smem, int nitems) {
 
 void launch_yinv(const YInvJobList& jobs, const YPassArgs& a, cudaStream_t s) {
     if (jobs.n <= 0) return;
-    if (launch_yinv_warp(jobs, a, s)) return;
+    if (launch_yinv_column(jobs, a, s) || launch_yinv_warp(jobs, a, s)) return;
     if (a.f32) throw std::runtime_error("mixed precision: y transform length has no warp plan");
     const int nch = (a.kxc + KC - 1) / KC;
     const int nitems = jobs.n * a.nzp * nch;
@@ -368,7 +368,7 @@ void launch_yinv(const YInvJobList& jobs, const YPassArgs& a, cudaStream_t s) {
 
 void launch_yfwd(const YFwdJobList& jobs, const YPassArgs& a, cudaStream_t s) {
     if (jobs.n <= 0) return;
-    if (launch_yfwd_warp(jobs, a, s)) return;
+    if (launch_yfwd_column(jobs, a, s) || launch_yfwd_warp(jobs, a, s)) return;
     if (a.f32) throw std::runtime_error("mixed precision: y transform length has no warp plan");
     const int nch = (a.kxc + KC - 1) / KC;
     const int nitems = jobs.n * a.nzp * nch;

@@ -153,41 +153,44 @@ __device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, int f, const do
                 }
             }
         } else {
+            // the thread's two columns as 16-byte accesses (C and cb are even: cb < C covers both):
+            // 8-byte stores of every second double wrote each sector twice
+            if (cb >= g.C) return;
+            double* __restrict__ o = out + (long long)(t0 * 16 + gq + g.roff) * g.C + cb;
+            const double* __restrict__ ro = (E == EPI_POISSON_RHS) ? aux + (o - out) : o;
+            const long long r8 = 8 * g.C;
 #pragma unroll
-        for (int t = 0; t < NTL; ++t) {
-            // the field values this tile's epilogue reads, loaded together before its stores
-            double old[4] = {0.0, 0.0, 0.0, 0.0};
-            if (RD && (E == EPI_POISSON_RHS || g.beta != 0.0)) {
+            for (int t = 0; t < NTL; ++t) {
+                // the field values this tile's epilogue reads, loaded together before its stores
+                double2 old[2];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int r = (t0 + t) * 16 + (q >> 1) * 8 + gq;
-                    const long long c = cb + (q & 1);
-                    if (r < rend && c < g.C) {
-                        const long long o = (long long)(r + g.roff) * g.C + c;
-                        old[q] = (E == EPI_POISSON_RHS) ? aux[o] : out[o];
+                for (int hh = 0; hh < 2; ++hh) {
+                    old[hh] = make_double2(0.0, 0.0);
+                    if (RD && (E == EPI_POISSON_RHS || g.beta != 0.0) && (t0 + t) * 16 + hh * 8 + gq < rend)
+                        old[hh] = *reinterpret_cast<const double2*>(ro + (2 * t + hh) * r8);
+                }
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int r = t * 16 + hh * 8 + gq;
+                    if (t0 * 16 + r >= rend) continue;
+                    double v[2] = {acc[t][2 * hh], acc[t][2 * hh + 1]};
+                    const double ov[2] = {old[hh].x, old[hh].y};
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        if constexpr (E == EPI_AXPBY) {
+                            v[e] = g.alpha * v[e] + (g.beta != 0.0 ? g.beta * ov[e] : 0.0);
+                        } else if constexpr (E == EPI_HELM_SCALE) {
+                            const double dfac = (-ew2[e]) - g.sigma;
+                            v[e] = v[e] / (erow[r] + dfac);
+                        } else if constexpr (E == EPI_POISSON_RHS) {
+                            v[e] = -v[e] - ew2[e] * ov[e];
+                        } else if constexpr (E == EPI_LIFT_ADD) {  // acc + hb*bcb + ht*bct
+                            if (bcb != nullptr) v[e] = v[e] + erow[r] * eb[e] + erow[er + r] * et[e];
+                        }
                     }
+                    *reinterpret_cast<double2*>(o + (2 * t + hh) * r8) = make_double2(v[0], v[1]);
                 }
             }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int r = (t0 + t) * 16 + (q >> 1) * 8 + gq;
-                const int e = q & 1;
-                const long long c = cb + e;
-                if (r >= rend || c >= g.C) continue;
-                double v = acc[t][q];
-                if constexpr (E == EPI_AXPBY) {
-                    v = g.alpha * v + (g.beta != 0.0 ? g.beta * old[q] : 0.0);
-                } else if constexpr (E == EPI_HELM_SCALE) {
-                    const double dfac = (-ew2[e]) - g.sigma;
-                    v = v / (erow[r - t0 * 16] + dfac);
-                } else if constexpr (E == EPI_POISSON_RHS) {
-                    v = -v - ew2[e] * old[q];
-                } else if constexpr (E == EPI_LIFT_ADD) {  // acc + hb*bcb + ht*bct
-                    if (bcb != nullptr) v = v + erow[r - t0 * 16] * eb[e] + erow[er + r - t0 * 16] * et[e];
-                }
-                out[(long long)(r + g.roff) * g.C + c] = v;
-            }
-        }
         }
     };
     switch (g.epi) {

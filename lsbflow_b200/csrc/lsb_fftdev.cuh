@@ -57,7 +57,7 @@ __device__ __forceinline__ V omega(int m) {
 
 // R-point DFT in registers: 2, 3, 4 directly, 5 and 7 from the sums and differences of the
 // pairs (j, R - j), 9 = 3 x 3 and 6, 8, 12, 16 = A*B (A in {4,3}) by one four-step split with
-// constant twiddles, 10, 14 and 15 = A*B with coprime factors by the prime-factor map (input
+// constant twiddles, 10, 14, 15, 18, 20 and 24 = A*B with coprime factors by the prime-factor map (input
 // B a + A b, output k = ka mod A = kb mod B), which needs no twiddles.
 template <int R, int SIGN, class V>
 __device__ __forceinline__ void dft_reg(V (&v)[R]) {
@@ -117,8 +117,8 @@ __device__ __forceinline__ void dft_reg(V (&v)[R]) {
             v[k] = cadd(e, o);
             v[R - k] = csub(e, o);
         }
-    } else if constexpr (R == 10 || R == 14 || R == 15) {
-        constexpr int A = (R % 2 == 0) ? 2 : 3, B = R / A;
+    } else if constexpr (R == 10 || R == 14 || R == 15 || R == 18 || R == 20 || R == 24) {
+        constexpr int A = (R == 20) ? 4 : ((R == 15 || R == 24) ? 3 : 2), B = R / A;
         V w[B][A];
 #pragma unroll
         for (int b = 0; b < B; ++b) {

@@ -101,6 +101,7 @@ struct YPassArgs {
     FftPlan plan;               // length nyl
     int f32 = 0;                // 1: y-intermediates in FP32, transforms in FP32 (mixed form)
     int y_tma = 0;              // FP64 tiles staged by TMA tile loads (1) or by cp.async (0)
+    int column = 1;             // FP64: the column-per-thread pass where the length has one
     int* err = nullptr;         // raised when a bounded wait of a TMA-staged pass timed out
 };
 
@@ -178,6 +179,11 @@ struct NlRowArgs {
     const double* lamx;   // [nxl] fringe lambda(x) or nullptr (only on the unpadded grid)
 };
 void launch_row_nl(const NlRowArgs& a, cudaStream_t s);
+
+// spanwise passes of short lengths, a column per thread (fft_column.cu); false when the length
+// has none
+bool launch_yinv_column(const YInvJobList& jobs, const YPassArgs& a, cudaStream_t s);
+bool launch_yfwd_column(const YFwdJobList& jobs, const YPassArgs& a, cudaStream_t s);
 
 // warp-group register FFT variants (fft_warp.cu); they return false when the plan has no
 // warp split, in which case the block-batched kernels of fft_kernels.cu run instead

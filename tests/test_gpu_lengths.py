@@ -59,6 +59,22 @@ def test_product_rows(nx, ny, over):
     s.close()
 
 
+@pytest.mark.parametrize("layout", ["correct", "ref"])
+@pytest.mark.parametrize("ny", [4, 6, 8, 12, 16, 20, 24, 32, 36, 48, 64, 72, 80, 96, 112, 128])
+def test_forcing_accumulates_over_every_spanwise_split(ny, layout):
+    # the fringe forcing of padded runs is added to N by the forward spanwise pass
+    from lsbflow_b200 import lib
+    st = hs.make_setup(workload("dns64", nx=64, ny=ny, nz=5, dealiasflag=1, dealias_layout=layout, forcing=1))
+    s = lib.Solver(st)
+    rng = np.random.default_rng(ny)
+    u = [rng.standard_normal((6, ny, 64)) for _ in range(3)]
+    O.norm(u, ny)
+    got, ref = s.nlterm(np.array(u)), O.nlterm_skewsym(st, u)
+    for l in range(3):
+        assert rel(got[l], ref[l]) < TOL_OP, l
+    s.close()
+
+
 def test_mixed_form_takes_the_lengths_it_took():
     # the register counts that only FP64 has do not open the mixed form to new lengths
     from lsbflow_b200 import lib
