@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(256, 2) k_row_nl(NlRowArgs a) {
 }
 
 void launch_row_nl(const NlRowArgs& a, cudaStream_t s) {
-    if (launch_row_nl_warp(a, s)) return;
+    if (launch_row_nl_twelve(a, s) || launch_row_nl_warp(a, s)) return;
     if (a.r.f32) throw std::runtime_error("mixed precision: x transform length has no warp plan");
     const size_t sm = (size_t)36 * a.r.rp.half.ls * sizeof(double2);
     const int nitems = a.r.nyl * a.r.nzp;

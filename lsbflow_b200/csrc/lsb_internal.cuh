@@ -179,6 +179,9 @@ struct NlRowArgs {
     const double* lamx;   // [nxl] fringe lambda(x) or nullptr (only on the unpadded grid)
 };
 void launch_row_nl(const NlRowArgs& a, cudaStream_t s);
+// FP64 product rows of 384 complex values (row_products.cu); false for other lengths, and where the
+// row's modes do not fit shared memory (the unpadded 768-point grid)
+bool launch_row_nl_twelve(const NlRowArgs& a, cudaStream_t s);
 
 // spanwise passes of short lengths, a column per thread (fft_column.cu); false when the length
 // has none

@@ -59,6 +59,20 @@ def test_product_rows(nx, ny, over):
     s.close()
 
 
+def test_product_rows_of_384_modes_over_several_rows_per_warp():
+    # 144 x 13 rows on 148 blocks of 7 warps: every warp stages its next row, some have one, some two
+    from lsbflow_b200 import lib
+    st = hs.make_setup(workload("dns64", nx=512, ny=96, nz=12, dealiasflag=1, forcing=0))
+    s = lib.Solver(st)
+    rng = np.random.default_rng(0)
+    u = [rng.standard_normal((13, 96, 512)) for _ in range(3)]
+    O.norm(u, 96)
+    got, ref = s.nlterm(np.array(u)), O.nlterm_skewsym(st, u)
+    for l in range(3):
+        assert rel(got[l], ref[l]) < TOL_OP, l
+    s.close()
+
+
 @pytest.mark.parametrize("layout", ["correct", "ref"])
 @pytest.mark.parametrize("ny", [4, 6, 8, 12, 16, 20, 24, 32, 36, 48, 64, 72, 80, 96, 112, 128])
 def test_forcing_accumulates_over_every_spanwise_split(ny, layout):
