@@ -99,8 +99,9 @@ __global__ void __launch_bounds__(32 * ycol_warps(T), ycol_blocks(V, T, ACC))
         }
     };
     auto kept = [&](int o) { return act && (INV || unpad_row_c(o, ny, N, a.layout) >= 0); };
+    const double2* prev = ACC ? reinterpret_cast<const double2*>(fj.j[jb].prev) + (long long)z * rows_out * h + c : nullptr;
     auto previous = [&](int o) {
-        return (ACC && beta != 0.0 && kept(o)) ? out[(long long)unpad_row_c(o, ny, N, a.layout) * h] : zero;
+        return (ACC && beta != 0.0 && kept(o)) ? prev[(long long)unpad_row_c(o, ny, N, a.layout) * h] : zero;
     };
     auto mirror = [&](int o) {  // the row that the Hermitian symmetrisation pairs with o
         return pad_row_c((ny - unpad_row_c(o, ny, N, a.layout)) % ny, ny, N, a.layout);

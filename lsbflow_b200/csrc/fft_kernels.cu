@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(256, 2) k_yfwd(YFwdJobList jobs, YPassArgs a, 
             double2* o = reinterpret_cast<double2*>(job.out + ((long long)z * ny + j) * a.nx + 2 * c);
             double2 r;
             if (job.beta != 0.0) {
-                const double2 old = *o;
+                const double2 old = *reinterpret_cast<const double2*>(job.prev + ((long long)z * ny + j) * a.nx + 2 * c);
                 r = make_double2(fma(job.alpha, v.x, job.beta * old.x), fma(job.alpha, v.y, job.beta * old.y));
             } else {
                 r = make_double2(job.alpha * v.x, job.alpha * v.y);

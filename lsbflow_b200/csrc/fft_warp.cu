@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(256, R <= 8 ? 4 : (R <= 9 ? 3 : 2)) k_ywarp(YI
                     const int j = idx / WKC, cc = idx - j * WKC, c = c0 + cc;
                     old[e] = make_double2(0.0, 0.0);
                     if (job.beta != 0.0 && idx < ny * WKC && c < a.kxc)
-                        old[e] = *reinterpret_cast<const double2*>(job.out + ((long long)z * ny + j) * a.nx + 2 * c);
+                        old[e] = *reinterpret_cast<const double2*>(job.prev + ((long long)z * ny + j) * a.nx + 2 * c);
                 }
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
@@ -1499,7 +1499,7 @@ __global__ void __launch_bounds__(256, 4) k_ywarp_f(YInvJobList ij, YFwdJobList 
                     const int j = idx / WKC, cc = idx - j * WKC, c = c0 + cc;
                     old[e] = make_double2(0.0, 0.0);
                     if (job.beta != 0.0 && idx < ny * WKC && c < a.kxc)
-                        old[e] = *reinterpret_cast<const double2*>(job.out + ((long long)z * ny + j) * a.nx + 2 * c);
+                        old[e] = *reinterpret_cast<const double2*>(job.prev + ((long long)z * ny + j) * a.nx + 2 * c);
                 }
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {

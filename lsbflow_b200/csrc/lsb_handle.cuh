@@ -193,10 +193,12 @@ void diag_compute(lsb_handle* h, lsb_diagnostics* out);
 // lam / lmeans / nlam: the first nlam fields enter as the fringe forcing lambda(x) (m - q),
 // m = lmeans[i][z] (or 0), formed by the row transform as it reads them.  tau: the last six
 // fields are the dynamic model's stresses, formed and transformed by the fused row pass from
-// its inputs (their phys entries are not read)
+// its inputs (their phys entries are not read).  prev: the fields that beta scales (the spec
+// fields themselves when null)
 void phys_to_spec(lsb_handle* h, const double* const* phys, double* const* spec, int nf, int nzp, double alpha,
                   double beta, double* const* ybuf, bool f32 = false, const double* lam = nullptr,
-                  const double* const* lmeans = nullptr, int nlam = 0, const TauRowArgs* tau = nullptr);
+                  const double* const* lmeans = nullptr, int nlam = 0, const TauRowArgs* tau = nullptr,
+                  const double* const* prev = nullptr);
 void spec_to_phys(lsb_handle* h, const double* const* spec, double* const* phys, int nf, int nzp,
                   const double* const* means, const int* modes, bool f32 = false, double scale = 1.0);
 void zgemm(lsb_handle* h, const Mat& m, const double* in, double* out, int nf, int epi, double alpha, double beta,

@@ -87,9 +87,10 @@ struct YInvJob {
 struct YFwdJob {
     const double* in;   // y-intermediate [nzp][nyl][nx]
     double* out;        // spectral [nzp][ny][nx]
-    double alpha;       // out = alpha * T(in) + beta * out
+    double alpha;       // out = alpha * T(in) + beta * prev
     double beta;
     int sym;            // apply the kx = 0 Hermitian symmetrisation of the horfft round trip
+    const double* prev; // the field added to (read where beta != 0); it may be out itself
 };
 
 struct YPassArgs {

@@ -332,7 +332,7 @@ namespace lsb {
 // horfft(-1): physical (unpadded, [nzp][ny][nx]) -> spectral, nf fields
 void phys_to_spec(lsb_handle* h, const double* const* phys, double* const* spec, int nf, int nzp, double alpha,
                   double beta, double* const* ybuf, bool f32, const double* lam, const double* const* lmeans,
-                  int nlam, const TauRowArgs* tau) {
+                  int nlam, const TauRowArgs* tau, const double* const* prev) {
     if (tau && (nf > kMaxJobs || nf < 6)) fail(LSB_ERR_STATE, "fused stress pass: 6..12 fields in one batch");
     for (int f0 = 0; f0 < nf; f0 += kMaxJobs) {
         const int n = std::min(kMaxJobs, nf - f0);
@@ -348,7 +348,7 @@ void phys_to_spec(lsb_handle* h, const double* const* phys, double* const* spec,
                 rj.j[i].mean = m;
                 rj.j[i].add_mean = m ? 1.0 : 0.0;
             }
-            yj.j[i] = YFwdJob{y, spec[f0 + i], alpha, beta, 0};
+            yj.j[i] = YFwdJob{y, spec[f0 + i], alpha, beta, 0, prev ? prev[f0 + i] : spec[f0 + i]};
         }
         RowArgs ra = rowargs(h, false, nzp);
         YPassArgs ya = ypass(h, false, nzp);
@@ -451,8 +451,8 @@ void nlterm(lsb_handle* h, const double* uin, double* Nout) {
     { TimerScope ts(h, "row_nl"); launch_row_nl(na, h->stream); }
     YFwdJobList yf{};
     yf.n = 9;
-    for (int l = 0; l < 3; ++l) yf.j[l] = YFwdJob{na.N[l], Nout + l * S, 1.0, 0.0, dealias ? 1 : 0};
-    for (int m = 0; m < 6; ++m) yf.j[3 + m] = YFwdJob{na.H[m], h->H + m * S, 1.0, 0.0, dealias ? 1 : 0};
+    for (int l = 0; l < 3; ++l) yf.j[l] = YFwdJob{na.N[l], Nout + l * S, 1.0, 0.0, dealias ? 1 : 0, nullptr};
+    for (int m = 0; m < 6; ++m) yf.j[3 + m] = YFwdJob{na.H[m], h->H + m * S, 1.0, 0.0, dealias ? 1 : 0, nullptr};
     { TimerScope ts(h, "yfwd_nl"); launch_yfwd(yf, ya, h->stream); }
     if (f32nl) launch_add_half_sq(h->H, h->ubar, d.C(), d.nzp, h->stream);
 
@@ -1769,7 +1769,7 @@ int lsb_dealias_product(lsb_handle* h, const double* a, const double* b, double*
         launch_row_r2c(rf, rowargs(h, true, d.nzp), h->stream);
         YFwdJobList yf{};
         yf.n = 1;
-        yf.j[0] = YFwdJob{h->Y, h->io + 2 * S, 1.0, 0.0, 0};
+        yf.j[0] = YFwdJob{h->Y, h->io + 2 * S, 1.0, 0.0, 0, nullptr};
         launch_yfwd(yf, ypass(h, true, d.nzp), h->stream);
         const double* ss2[1] = {h->io + 2 * S};
         double* pp2[1] = {h->phys + 2 * h->P};
