@@ -49,14 +49,22 @@ __global__ void k_specfilter(SpecFilterArgs a) {
 // ---------------------------------------------------------------- velocity RHS
 // rhs_l = -dtnui*(dt*(ab0 N + ab1 nln + ab2 nlnm) + bdf0 u + bdf1 un + bdf2 unm) ;
 // rhs_1 -= horfft(ubarpp) (the (0,0) mode)      src/navierstokes.f90:1239,1282-1296
+// Bound by DRAM (18 fields in, 3 out): 16-byte accesses, a block of modes per component, the plane
+// index by 32-bit division (S < 2^31, checked at create) and only where the mean mode asks for it.
 __global__ void k_rhs(RhsArgs a) {
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < 3 * a.S; e += (long long)gridDim.x * blockDim.x) {
-        const int l = (int)(e / a.S);
-        const long long x = e % a.S;
-        const double nlt = a.ab[0] * a.N[l][x] + a.ab[1] * a.nln[l][x] + a.ab[2] * a.nlnm[l][x];
-        double r = -a.dtnui * (a.dt * nlt + a.bdf[0] * a.u[l][x] + a.bdf[1] * a.un[l][x] + a.bdf[2] * a.unm[l][x]);
-        if (l == 0 && (x % a.C) == 0) r = r - a.ubarpp[x / a.C];
-        a.rhs[l][x] = r;
+    const int l = blockIdx.y;
+    const unsigned n2 = (unsigned)(a.S / 2), c2 = (unsigned)(a.C / 2);
+    auto at = [&](const double* f, unsigned e) { return reinterpret_cast<const double2*>(f)[e]; };
+    auto value = [&](double n0, double n1, double n2_, double u0, double u1, double u2) {
+        const double nlt = a.ab[0] * n0 + a.ab[1] * n1 + a.ab[2] * n2_;
+        return -a.dtnui * (a.dt * nlt + a.bdf[0] * u0 + a.bdf[1] * u1 + a.bdf[2] * u2);
+    };
+    for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n2; e += gridDim.x * blockDim.x) {
+        const double2 n0 = at(a.N[l], e), n1 = at(a.nln[l], e), m2 = at(a.nlnm[l], e);
+        const double2 u0 = at(a.u[l], e), u1 = at(a.un[l], e), u2 = at(a.unm[l], e);
+        double2 r = make_double2(value(n0.x, n1.x, m2.x, u0.x, u1.x, u2.x), value(n0.y, n1.y, m2.y, u0.y, u1.y, u2.y));
+        if (l == 0 && e % c2 == 0) r.x = r.x - a.ubarpp[e / c2];
+        reinterpret_cast<double2*>(a.rhs[l])[e] = r;
     }
 }
 
@@ -261,7 +269,10 @@ static inline int nblk(long long n) {
 }
 
 void launch_specfilter(const SpecFilterArgs& a, cudaStream_t s) { lsb::note_launch(); k_specfilter<<<nblk(3 * a.S / 2), 256, 0, s>>>(a); }
-void launch_rhs(const RhsArgs& a, cudaStream_t s) { lsb::note_launch(); k_rhs<<<nblk(3 * a.S), 256, 0, s>>>(a); }
+void launch_rhs(const RhsArgs& a, cudaStream_t s) {
+    lsb::note_launch();
+    k_rhs<<<dim3(nblk(a.S / 2), 3), 256, 0, s>>>(a);
+}
 void launch_bc_planes(const BcArgs& a, cudaStream_t s) {
     lsb::note_launch();
     k_bc_planes<<<(unsigned)((a.C / 2 + BC_MODES - 1) / BC_MODES), BC_MODES * BC_SLICES, 0, s>>>(a);
