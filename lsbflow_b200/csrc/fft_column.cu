@@ -228,7 +228,8 @@ bool dispatch(const YInvJobList& ij, const YFwdJobList& fj, const YPassArgs& a, 
         LSB_YC(7, 4) LSB_YC(10, 3) LSB_YC(8, 4) LSB_YC(9, 4) LSB_YC2(8, 5, 10, 4) LSB_YC(7, 6) LSB_YC2(8, 6, 12, 4)
         LSB_YC(9, 6) LSB_YC(8, 7) LSB_YC2(10, 6, 12, 5) LSB_YC(8, 8) LSB_YC2(9, 8, 12, 6) LSB_YC(10, 8)
         LSB_YC(12, 7) LSB_YC(10, 9) LSB_YC2(8, 12, 12, 8) LSB_YC(12, 9) LSB_YC(14, 8) LSB_YC2(10, 12, 12, 10)
-        LSB_YC(16, 8) LSB_YC(12, 12) LSB_YC(16, 12)
+        LSB_YC(16, 8) LSB_YC(12, 12) LSB_YC(16, 12) LSB_YC(7, 3) LSB_YC(5, 5) LSB_YC(9, 3) LSB_YC(7, 5) LSB_YC(9, 5)
+        LSB_YC(9, 7)
 #undef LSB_YC
 #undef LSB_YC2
         default: return false;

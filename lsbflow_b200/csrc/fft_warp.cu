@@ -298,6 +298,8 @@ struct alignas(64) YTmaMaps {
 };
 
 // ----------------------------------------------------------------------------- spanwise
+// The tiled pass: lengths that fft_column.cu has no split for (above 144, mostly), the sigma model's
+// gradients, and (k_ywarp_f below) the mixed form.
 // One kernel for both directions.  Work item = (job, z, chunk of WKC kx columns); the tile
 // [nyl][WKC] is staged double-buffered -- by cp.async (TMA = false) or by TMA tile loads that
 // complete on an mbarrier per buffer (TMA = true, 2 or 4 box loads issued by one thread) --,
@@ -1665,16 +1667,6 @@ void ylaunch(const YInvJobList& ij, const YFwdJobList& fj, const YPassArgs& a, c
     if (a.plan.g == 16) {
         use_tma ? go(k_ywarp<R, INV, 16, true>) : go(k_ywarp<R, INV, 16>);
         return;
-    }
-    if constexpr (R % 2 == 1 && R > 1) {  // (groups of 8 and 4 lanes come with an odd R)
-        if (a.plan.g == 8) {
-            use_tma ? go(k_ywarp<R, INV, 8, true>) : go(k_ywarp<R, INV, 8>);
-            return;
-        }
-        if (a.plan.g == 4 && !use_tma) {
-            go(k_ywarp<R, INV, 4>);
-            return;
-        }
     }
     use_tma ? go(k_ywarp<R, INV, 0, true>) : go(k_ywarp<R, INV>);
 }

@@ -74,7 +74,7 @@ def test_product_rows_of_384_modes_over_several_rows_per_warp():
 
 
 @pytest.mark.parametrize("layout", ["correct", "ref"])
-@pytest.mark.parametrize("ny", [4, 6, 8, 12, 16, 20, 24, 32, 36, 48, 64, 72, 80, 96, 112, 128])
+@pytest.mark.parametrize("ny", [4, 6, 8, 12, 14, 16, 18, 20, 24, 30, 42, 32, 36, 48, 64, 72, 80, 96, 112, 128])
 def test_forcing_accumulates_over_every_spanwise_split(ny, layout):
     # the fringe forcing of padded runs is added to N by the forward spanwise pass
     from lsbflow_b200 import lib
