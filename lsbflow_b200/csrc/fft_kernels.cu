@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(256, 2) k_row_r2c(RowJobList jobs, RowArgs a) 
 
 void launch_row_c2r(const RowJobList& jobs, const RowArgs& a, cudaStream_t s) {
     if (jobs.n <= 0) return;
-    if (launch_row_c2r_warp(jobs, a, s)) return;
+    if (launch_row_split(jobs, a, s, true) || launch_row_c2r_warp(jobs, a, s)) return;
     if (a.f32) throw std::runtime_error("mixed precision: x transform length has no warp plan");
     const int nitems = jobs.n * ((a.nyl * a.nzp + RB - 1) / RB);
     const size_t sm = (size_t)3 * RB * a.rp.half.ls * sizeof(double2);
@@ -554,7 +554,7 @@ void launch_row_r2c(const RowJobList& jobs, const RowArgs& a, cudaStream_t s) {
             return;
         }
     }
-    if (launch_row_r2c_warp(jobs, a, s)) return;
+    if (launch_row_split(jobs, a, s, false) || launch_row_r2c_warp(jobs, a, s)) return;
     launch_row_r2c_batched(jobs, a, s);
 }
 

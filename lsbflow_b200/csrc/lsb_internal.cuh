@@ -129,10 +129,12 @@ struct RowArgs {
     long long row_pitch;        // physical row pitch in doubles (nxl)
     const double* wavx;
     RealPlan rp;
+    int split = 1;              // FP64: the two-step split where the length has one (fft_rows.cu)
 };
 struct RowJobList { int n; RowIO j[kMaxJobs]; };
 void launch_row_c2r(const RowJobList& jobs, const RowArgs& a, cudaStream_t s);
 void launch_row_r2c(const RowJobList& jobs, const RowArgs& a, cudaStream_t s);
+bool launch_row_split(const RowJobList& jobs, const RowArgs& a, cudaStream_t s, bool c2r);
 
 // the unpadded row pass of the dynamic SGS model's physical fields, with the model's first
 // pointwise pass fused in: u_l, S_ij and delta^2 |S| S_ij from the y-intermediates

@@ -323,6 +323,9 @@ RowArgs rowargs(lsb_handle* h, bool padded, int nzp) {
     r.row_pitch = r.nxl;
     r.wavx = h->wavx;
     r.rp = padded ? h->rxl : h->rx;
+    // the sigma model's gradients keep the lane networks' roundings, as in ypass, and so do the FP64
+    // rows of the mixed form (the split gives its step nothing: 1259 us at 256 x 64 x 129 either way)
+    r.split = h->cfg.precision == 0 && !(h->cfg.sgsflag == 1 && h->cfg.sgsmodel == 2 && !padded);
     return r;
 }
 

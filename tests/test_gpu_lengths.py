@@ -20,8 +20,8 @@ TOL_OP = 1e-12
 
 # (nx, ny): half and padded half lengths nx/2, 3 nx/4 and spanwise ny, 3 ny/2
 GRIDS = [(20, 4), (24, 6), (28, 10), (36, 12), (40, 14), (48, 18), (56, 20), (60, 28), (64, 30), (72, 36), (80, 40),
-         (96, 48), (112, 56), (120, 60), (144, 80), (160, 6), (192, 96), (224, 8), (240, 16), (288, 4), (320, 10),
-         (384, 24), (448, 4), (512, 20)]
+         (96, 48), (112, 56), (120, 60), (128, 14), (144, 80), (160, 6), (192, 96), (224, 8), (240, 16),
+         (256, 6), (288, 4), (320, 10), (384, 24), (448, 4), (512, 20)]
 
 
 def rel(a, b):
